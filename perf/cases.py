@@ -250,6 +250,7 @@ def draw(rng):
             most, fp32 = 1e7, False
         elif option < 0.45:
             nsplit, inflight, scale = rng.choice((4, 8, 16)), 2_000_000, 0.5
+            most = 6e7 / nsplit
     elif kind == "history":
         most, scale = 1.2e7, 1.2
     scale *= max(1, jobs)
