@@ -166,22 +166,6 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kMinBlocks) transport_ke
 // ---------------------------------------------------------------------------
 template <typename R>
 struct Wavefront {
-  R *ph_f[2];
-  int *ph_k[2];
-  R *el_f[2];
-  int *el_k[2];
-  int *ph_s[2], *el_s[2]; // tally slot per queued particle (beamlet jobs), else null
-  R *ei_f[2];             // electrons waiting for a discrete interaction
-  int *ei_k[2];
-  int *ei_s[2];
-  R *pi_f[2];             // photons waiting for their interaction
-  int *pi_k[2];
-  int *pi_s[2];
-  R *ph_t[2];             // photon flights: mean free paths left (-1: a new flight)
-  unsigned cap;           // slots per queue
-  unsigned *ctr;          // queue counters (queue_ctr(): photon, electron, electron-interaction,
-                          // photon-interaction and boundary-electron, three rotation slots each;
-                          // boundary electrons fill the electron queue from the top)
   unsigned long long *work;      // [3] chunk counters of the phase, kCounterPad words apart
   unsigned long long *injected;  // [2] histories injected before the iteration
   unsigned *bar_arrive;
@@ -203,20 +187,6 @@ struct Wavefront {
 };
 
 constexpr int kDefaultChunkEvents = 1;
-
-// Every counter of the schedule has an L2 line of its own, kCounterPad words
-// apart.  All warps append to the same few queues, so the counters are the
-// hottest addresses of the run (21 atomics per history against 46 deposits
-// spread over the tallies), and one L2 line serves about one atomic per
-// clock: side by side in one line, as they were, they bounded the kernel
-// whatever its occupancy or instruction count.
-// Measured, lines apart against side by side: 6 MV slab (2 mm, 10x10 cm2,
-// 1e8 histories, FP32) 1061 -> 959 ms; a 250 kVp job of 6e6 histories 9.1 ->
-// 7.9 ms; FP64 jobs unchanged within their spread.
-constexpr int kCounterPad = 64;
-enum { CTR_PH = 0, CTR_EL, CTR_EI, CTR_PI, CTR_EB, CTR_KINDS };
-// Counter of queue kind q in rotation slot c (0..2).
-__device__ __forceinline__ unsigned *queue_ctr(unsigned *ctr, int q, int c) { return ctr + (3 * q + c) * kCounterPad; }
 
 // End-of-run drain: once every history is injected and fewer than
 // kDrainPerWarp particles per 32 threads are in flight, the GPU is short
@@ -304,7 +274,6 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
   L.rng.i = P.rng_ijc[gtid];
   L.rng.j = P.rng_ijc[P.nlanes + gtid];
   L.rng.c = P.rng_ijc[2 * P.nlanes + gtid];
-  L.queue_cap = W.cap;
   // Photon and discrete electron interactions run in their own chunks
   // (measured on the 6 MV slab: electrons FP32 2.85e7 -> 3.10e7 and FP64
   // 2.02e6 -> 2.22e6 hist/s; photons then 3.96e7 -> 4.29e7).
@@ -319,12 +288,12 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
     // A counter counts the appends that did not fit too (they set
     // ERR_QUEUE): the reads below stay inside the queues.  The two ends of
     // the electron queue must not have met, else records were overwritten.
-    const unsigned n_ph = min(vload(queue_ctr(W.ctr, CTR_PH, cin)), W.cap);
-    const unsigned n_el = min(vload(queue_ctr(W.ctr, CTR_EL, cin)), W.cap);
-    const unsigned n_ei = min(vload(queue_ctr(W.ctr, CTR_EI, cin)), W.cap);
-    const unsigned n_pi = min(vload(queue_ctr(W.ctr, CTR_PI, cin)), W.cap);
-    const unsigned n_eb = min(vload(queue_ctr(W.ctr, CTR_EB, cin)), W.cap - n_el);
-    if (gtid == 0 && static_cast<unsigned long long>(vload(queue_ctr(W.ctr, CTR_EL, cin))) + vload(queue_ctr(W.ctr, CTR_EB, cin)) > W.cap)
+    const unsigned n_ph = min(vload(queue_ctr(P.q.ctr, QUEUE_PH, cin)), P.q.cap);
+    const unsigned n_el = min(vload(queue_ctr(P.q.ctr, QUEUE_EL, cin)), P.q.cap);
+    const unsigned n_ei = min(vload(queue_ctr(P.q.ctr, QUEUE_EI, cin)), P.q.cap);
+    const unsigned n_pi = min(vload(queue_ctr(P.q.ctr, QUEUE_PI, cin)), P.q.cap);
+    const unsigned n_eb = min(vload(queue_ctr(P.q.ctr, QUEUE_EB, cin)), P.q.cap - n_el);
+    if (gtid == 0 && static_cast<unsigned long long>(vload(queue_ctr(P.q.ctr, QUEUE_EL, cin))) + vload(queue_ctr(P.q.ctr, QUEUE_EB, cin)) > P.q.cap)
       L.err |= ERR_QUEUE;
     const unsigned long long injected = *static_cast<volatile unsigned long long *>(W.injected + bin);
     const long long remaining = P.nhist - static_cast<long long>(injected);
@@ -356,19 +325,15 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
       if (m > nfree) m = nfree > 0 ? nfree : 0;
     }
     if (gtid == 0) {
-      for (int q = 0; q < CTR_KINDS; q++) *queue_ctr(W.ctr, q, cfree) = 0;
+      for (int q = 0; q < QUEUE_KINDS; q++) *queue_ctr(P.q.ctr, q, cfree) = 0;
       W.work[cfree * (kCounterPad / 2)] = 0;
       W.injected[bout] = injected + static_cast<unsigned long long>(m);
     }
     // One phase: new histories, then photons, then electrons, each range
     // padded to a multiple of 32 so that a warp's chunk is one code path.
     // Everything produced goes to the next iteration's queues.
-    L.out = EmitTargets<R>{W.ph_f[bout], W.ph_k[bout], queue_ctr(W.ctr, CTR_PH, cout),
-                           W.el_f[bout], W.el_k[bout], queue_ctr(W.ctr, CTR_EL, cout),
-                           W.ph_s[bout], W.el_s[bout],
-                           W.ei_f[bout], W.ei_k[bout], queue_ctr(W.ctr, CTR_EI, cout), W.ei_s[bout],
-                           W.pi_f[bout], W.pi_k[bout], queue_ctr(W.ctr, CTR_PI, cout), W.pi_s[bout],
-                           queue_ctr(W.ctr, CTR_EB, cout), W.ph_t[bout]};
+    L.gen = bout;
+    L.slot_out = cout;
     // In the drain a flight runs to its end: the GPU is short of work and
     // every re-queued photon would cost an iteration.
     L.flight_cap = drain ? kNoFlightCap : W.flight_cap;
@@ -391,33 +356,29 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base >= total) break;
       const unsigned long long i = base + lane_id;
-      if (base >= r_in && base < r_in + ((static_cast<unsigned long long>(m) + 31) & ~31ull)) {
+      if (base >= r_in && base < r_ph) {
         const unsigned long long k = i - r_in;
         if (k < static_cast<unsigned long long>(m)) {
           L.init_history(static_cast<long long>(injected + k));
           if constexpr (HBH) L.hbh_start();
-          L.emit(L.p);
-          if constexpr (HBH) L.hbh_finish(0);
+          L.dest = L.p.iq == 0 ? QUEUE_PH : QUEUE_EL;
         }
-      } else if (base >= r_ph && base < r_ph + ph_pad) {
+      } else if (base >= r_ph && base < r_pi) {
         const unsigned long long k = i - r_ph;
         if (k < n_ph) {
-          L.take(W.ph_f[bin], W.ph_k[bin], static_cast<unsigned>(k), W.ph_s[bin]);
-          L.taken_mfp = __ldcg(W.ph_t[bin] + k);
+          L.take(QUEUE_PH, bin, static_cast<unsigned>(k));
           L.wf_photon_event();
           events++;
-          if constexpr (HBH) L.hbh_finish(1);
         }
-      } else if (base >= r_pi && base < r_pi + pi_pad) {
+      } else if (base >= r_pi && base < r_el) {
         const unsigned long long k = i - r_pi;
         if (k < n_pi) {
-          L.take(W.pi_f[bin], W.pi_k[bin], static_cast<unsigned>(k), W.pi_s[bin]);
+          L.take(QUEUE_PI, bin, static_cast<unsigned>(k));
           const bool survivor = L.p.iq == 2;
           L.p.iq = 0;
           L.deferred_photon_interaction(survivor);
-          if constexpr (HBH) L.hbh_finish(1);
         }
-      } else if (base >= r_el && base < r_eb + eb_pad) {
+      } else if (base >= r_el && base < r_ei) {
         // A chunk lies in one of the two electron ranges.
         const bool nb = base >= r_eb;
         const unsigned long long k = i - (nb ? r_eb : r_el);
@@ -428,8 +389,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
           // interaction queue if its step ended at a deferred interaction.
           // In the drain the interaction runs at once and the take goes on
           // with whatever electron is left on top.
-          L.take(W.el_f[bin], W.el_k[bin], nb ? W.cap - 1 - static_cast<unsigned>(k) : static_cast<unsigned>(k),
-                 W.el_s[bin]);
+          L.take(QUEUE_EL, bin, nb ? P.q.cap - 1 - static_cast<unsigned>(k) : static_cast<unsigned>(k));
           L.pending_interaction = false;
           int n = 0;
           do {
@@ -440,24 +400,24 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
               L.deferred_interaction();
             }
           } while (L.alive && !L.pending_interaction && L.p.iq != 0 && ++n < (drain ? kDrainSteps : W.chunk_events));
-          if (L.alive) {
-            if (L.pending_interaction) L.emit_pending();
-            else L.emit_step(L.p);
-          }
-          if constexpr (HBH) L.hbh_finish(1);
+          if (L.alive) L.dest = L.pending_interaction ? QUEUE_EI : L.step_queue();
         }
       } else {
         const unsigned long long k = i - r_ei;
         if (k < n_ei) {
-          L.take(W.ei_f[bin], W.ei_k[bin], static_cast<unsigned>(k), W.ei_s[bin]);
+          L.take(QUEUE_EI, bin, static_cast<unsigned>(k));
           L.deferred_interaction();
-          if (L.alive) L.emit(L.p);
-          if constexpr (HBH) L.hbh_finish(1);
+          if (L.alive) L.dest = L.p.iq == 0 ? QUEUE_PH : QUEUE_EL;
         }
       }
       // Every lane of the warp is here (a chunk is one code path): the warp
-      // merges the histories its lanes just completed.
-      if constexpr (HBH) L.hbh_warp_merge();
+      // appends what its lanes' events left and merges the histories they
+      // just completed.
+      L.flush();
+      if constexpr (HBH) {
+        L.hbh_finish(base < r_ph ? 0 : 1);
+        L.hbh_warp_merge();
+      }
     }
     bool bar_ok;
     if constexpr (HBH) bar_ok = grid_barrier(W.bar_arrive, W.bar_gen, gridDim.x, P.hbh.ctr, W.hbh_free + 2 * bout);
@@ -1114,7 +1074,7 @@ omc_status run_batches(omc_engine *e, PrecisionState<R> &S, const omc_run_config
 }
 
 struct WfCounters {
-  unsigned ctr[3 * CTR_KINDS * kCounterPad];
+  unsigned ctr[3 * QUEUE_KINDS * kCounterPad];
   unsigned long long work[3 * kCounterPad / 2];
   unsigned long long injected[kCounterPad / 2];  // [2]
   unsigned bar_arrive[kCounterPad], bar_gen[kCounterPad];  // [1] each
@@ -1170,45 +1130,22 @@ omc_status run_wavefront(omc_engine *e, PrecisionState<R> &S, const omc_run_conf
   unsigned long long cap = target * (4ull + 2ull * nsplit) + 4ull * nlanes;
   if (cap > 0x7fffffffull) cap = 0x7fffffffull;
   const bool hbh = cfg->history_stats != 0 && !(job && job->jobs);
-  const size_t tag_bytes = (job || hbh) ? static_cast<size_t>(cap) * sizeof(int) : 0;
-  size_t per_queue = static_cast<size_t>(cap) * (8 * sizeof(R) + sizeof(int)) + tag_bytes;
   // photons, electrons (those near a boundary from the top), electron and
-  // photon interactions; two generations each
-  const int nqueues = 8;
-  // and the photon flights' mean free paths left, two generations
-  const size_t mfp_bytes = (static_cast<size_t>(cap) * sizeof(R) + 255) & ~static_cast<size_t>(255);
-  if (S.queue.ensure(nqueues * per_queue + 2 * mfp_bytes) != OMC_OK) return OMC_ERR_NOMEM;
+  // photon interactions; two generations each, in blocks of 32 records
+  QueueLayout q{};
+  q.cap = static_cast<unsigned>((cap + 31) & ~31ull);
+  q.tags = (job || hbh) ? 1 : 0;
+  q.block = 32 * static_cast<unsigned>(8 * sizeof(R) + (1 + q.tags) * sizeof(int));
+  q.block_ph = q.block + 32 * static_cast<unsigned>(sizeof(R));
+  q.bytes = static_cast<unsigned long long>(q.cap / 32) * q.block;
+  q.bytes_ph = static_cast<unsigned long long>(q.cap / 32) * q.block_ph;
+  if (S.queue.ensure(2 * q.bytes_ph + 6 * q.bytes) != OMC_OK) return OMC_ERR_NOMEM;
   if (e->wf_counters.ensure(sizeof(WfCounters)) != OMC_OK) return OMC_ERR_NOMEM;
-  char *qb = static_cast<char *>(S.queue.p);
-  Wavefront<R> W{};
-  for (int q = 0; q < nqueues; q++) {
-    R *f = reinterpret_cast<R *>(qb + q * per_queue);
-    int *k = reinterpret_cast<int *>(qb + q * per_queue + static_cast<size_t>(cap) * 8 * sizeof(R));
-    int *tag = (job || hbh) ? k + cap : nullptr;
-    if (q < 2) {
-      W.ph_f[q] = f;
-      W.ph_k[q] = k;
-      W.ph_s[q] = tag;
-    } else if (q < 4) {
-      W.el_f[q - 2] = f;
-      W.el_k[q - 2] = k;
-      W.el_s[q - 2] = tag;
-    } else if (q < 6) {
-      W.ei_f[q - 4] = f;
-      W.ei_k[q - 4] = k;
-      W.ei_s[q - 4] = tag;
-    } else {
-      W.pi_f[q - 6] = f;
-      W.pi_k[q - 6] = k;
-      W.pi_s[q - 6] = tag;
-    }
-  }
-  W.ph_t[0] = reinterpret_cast<R *>(qb + nqueues * per_queue);
-  W.ph_t[1] = reinterpret_cast<R *>(qb + nqueues * per_queue + mfp_bytes);
-  W.flight_cap = kFlightCap<R>;
   WfCounters *wc = static_cast<WfCounters *>(e->wf_counters.p);
-  W.cap = static_cast<unsigned>(cap);
-  W.ctr = wc->ctr;
+  q.base = static_cast<char *>(S.queue.p);
+  q.ctr = wc->ctr;
+  Wavefront<R> W{};
+  W.flight_cap = kFlightCap<R>;
   W.work = wc->work;
   W.injected = wc->injected;
   W.bar_arrive = wc->bar_arrive;
@@ -1244,6 +1181,7 @@ omc_status run_wavefront(omc_engine *e, PrecisionState<R> &S, const omc_run_conf
   P.max_np = &dc->max_np;
   P.err = &dc->err;
   apply_job(P, S, job, e->nreg);
+  P.q = q;
   // History-by-history pool: a head block per history in flight plus
   // continuation blocks; an iteration keeps 4 blocks per thread back for
   // continuations.
