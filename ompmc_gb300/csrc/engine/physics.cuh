@@ -436,7 +436,10 @@ struct Lane {
     if (hblk < 0) return;
     const int delta = emitted - consumed;
     emitted = 0;
-    if (delta == 0) return;
+    if (delta == 0) {
+      hblk = -1;  // every lane comes here after a chunk, with or without a take
+      return;
+    }
     __threadfence();  // this lane's appends before the count
     const int left = atomicAdd(&P.hbh.blocks[hblk].live, delta) + delta;
     if (left == 0) {
