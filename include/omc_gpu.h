@@ -238,7 +238,8 @@ typedef enum omc_precision {
 typedef struct omc_run_config {
     long long nperbatch; /* histories per batch                           */
     int nbatch;          /* statistical batches (omc_dosxyz.c:1214-1225)  */
-    int ixx, jxx;        /* "rng seeds"; lane k uses the k-th seed pair   */
+    int ixx, jxx;        /* "rng seeds"; lane k (wavefront: warp k) uses the
+                            k-th seed pair                                */
     int nsplit;          /* "nsplit" photon splitting (ompmc.c:5964)      */
     int precision;       /* omc_precision                                 */
     int nlanes;          /* per-lane schedule: concurrent histories;

@@ -261,6 +261,7 @@ struct Params {
   // per-lane state in HBM
   int *rng_u;                // [97][nlanes]
   int *rng_ijc;              // [3][nlanes]
+  int *rng_w;                // wavefront: [kPoolWords][nlanes] warp streams
   R *stk;                    // [8][depth][nlanes]
   int *stk_key;              // [depth][nlanes]  ir*4 + iq+1
   // beamlet jobs: history h of the launch belongs to tally slot s with
@@ -384,6 +385,129 @@ __host__ __device__ inline void stream_seeds(int ixx, int jxx, long long k, int 
   const int c = (int)(lin % kJxxStreams);
   *jk = c == 0 ? kJxxStreams : c;
   *ik = (int)(((long long)(ixx - 1) + lin / kJxxStreams) % 31328) + 1;
+}
+
+// ---------------------------------------------------------------------------
+// RANMAR of the wavefront schedule: one stream per warp, 32 numbers a step.
+// The lagged sequence x[n] = x[n-97] - x[n-33] mod 2^24 only reaches back 33
+// numbers or more, so the 32 lanes of a converged warp produce 32
+// consecutive numbers of the stream at once, and each lane keeps what later
+// steps need: the values it produced 1 to 4 steps ago.  The numbers are those
+// of initRandom/getRandom (omc_random.c:58-187) for the warp's seed pair.
+// Which lane gets which number turns by kPoolTurn lanes a step.  Unturned,
+// the three numbers of one recurrence fell on two neighbouring lanes, whose
+// particles then made correlated choices (jobs of 2e5 histories: the total
+// energy 1.5% off, the voxels' mean z^2 1.7); turned, they fall on three
+// lanes (kPoolTurn * {1, 2, 3} avoid {1, 0, 1} mod 32), so any two lanes are
+// independent, as two RANMAR streams are.
+//
+// A lane takes its numbers from a stack of kPoolSlots in shared memory that
+// refill() tops up wherever the warp is converged (before every chunk and
+// every step of a drained track).  A draw in divergent code is then one
+// shared load instead of RANMAR's four loads, two stores and 30
+// instructions on a 97-word state per lane, and the shared memory per block
+// falls from 37 kB to 20 kB (FP32), which the L1 cache gets.
+//
+// An event has kPoolLow numbers to start with.  Its rejection loops, and
+// what follows them, ask for the numbers they are about to draw
+// (Lane::need); where a rejection loop has run the stack low, overflow()
+// adds numbers of a generator of the lane's own (PCG32, O'Neill,
+// HMC-CS-2014-0905), whose state is drawn from the warp's stream at launch.
+// (A call that carried on with a RANMAR stream per lane in device memory cost
+// 100 to 300 bytes of register spills around the call sites.)
+// Measured: 6 MV slab (2 mm, 1e8 histories) FP32 942 -> 806 ms, FP64 (1e7)
+// 1499 -> 1441 ms; slab on 1 cm voxels 116 -> 98 ms; positron field 55 -> 44
+// ms; nsplit 16 40 -> 34 ms; dij 116 -> 102 ms.
+constexpr int kPoolSlots = 32;     // numbers a lane's stack holds
+constexpr int kPoolLow = 26;       // refill() leaves every lane at least this many
+constexpr int kPoolSpill = 8;      // numbers overflow() adds
+constexpr int kWeylMod = 16777213, kWeylStep = 7654321;
+constexpr int kWeylStep32 = static_cast<int>(32ll * kWeylStep % kWeylMod);
+constexpr int kWeylStart = 362436;
+constexpr int kPoolWords = 5;      // saved words per lane: four past values, Weyl term
+constexpr int kPoolState = kPoolWords + 3;  // ... the turn of the next step, the overflow generator's state
+constexpr int kPoolTurn = 5;       // lanes a step's numbers are turned on by
+
+template <typename R>
+struct RngPool {
+  R *base;     // slot 0 of this lane's stack: slot k is base[32 * k]
+  int *state;  // the lane's words in shared memory, 32 apart: its values of
+               // the last four steps, the Weyl term of the last, the turn of
+               // the next step and the overflow generator's state
+  int n;       // numbers on the stack
+
+  __device__ __forceinline__ void restore(const int *w, int nlanes, int gl) {
+    n = 0;
+    for (int k = 0; k < kPoolWords; k++) state[32 * k] = w[static_cast<size_t>(k) * nlanes + gl];
+    state[32 * kPoolWords] = 0;
+    refill();
+    for (int k = kPoolWords + 1; k < kPoolState; k++) {  // 2 x 32 bits from 4 x 16
+      const unsigned hi = static_cast<unsigned>(base[32 * --n] * static_cast<R>(65536.0));
+      const unsigned lo = static_cast<unsigned>(base[32 * --n] * static_cast<R>(65536.0));
+      state[32 * k] = static_cast<int>(hi << 16 | lo);
+    }
+  }
+  __device__ __forceinline__ void save(int *w, int nlanes, int gl) const {
+    for (int k = 0; k < kPoolWords; k++) w[static_cast<size_t>(k) * nlanes + gl] = state[32 * k];
+  }
+  // Tops up the stacks of the warp; called by all 32 lanes together.
+  __device__ __forceinline__ void refill() {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, from = (lane - 1) & 31;
+    int k = __reduce_max_sync(full, kPoolLow - n);
+    if (k <= 0) return;
+    int v1 = state[0], v2 = state[32], v3 = state[64], v4 = state[96], c = state[128], turn = state[160];
+    do {
+      // x[n-33] and x[n-97]: the previous lane's value of the last step and
+      // of three steps ago (lane 0: lane 31's of one step earlier).
+      const int a = __shfl_sync(full, lane == 31 ? v2 : v1, from);
+      const int b = __shfl_sync(full, lane == 31 ? v4 : v3, from);
+      v4 = v3;
+      v3 = v2;
+      v2 = v1;
+      v1 = (b - a) & 0xffffff;
+      c -= kWeylStep32;
+      if (c < 0) c += kWeylMod;
+      const int u = __shfl_sync(full, (v1 - c) & 0xffffff, (lane + turn) & 31);
+      turn += kPoolTurn;
+      if (n < kPoolSlots) {
+        base[32 * n] = static_cast<R>(u) * static_cast<R>(1.0 / 16777216.0);
+        n++;
+      }
+    } while (--k > 0);
+    state[160] = turn & 31;
+    state[0] = v1;
+    state[32] = v2;
+    state[64] = v3;
+    state[96] = v4;
+    state[128] = c;
+  }
+  // More numbers for one lane, in divergent code.
+  __device__ __forceinline__ void overflow() {
+    unsigned long long x = static_cast<unsigned>(state[32 * kPoolWords + 32]) |
+                           static_cast<unsigned long long>(static_cast<unsigned>(state[32 * kPoolWords + 64])) << 32;
+#pragma unroll 1
+    for (int k = 0; k < kPoolSpill; k++) {
+      const unsigned r = static_cast<unsigned>(((x >> 18) ^ x) >> 27);
+      const unsigned out = __funnelshift_r(r, r, static_cast<unsigned>(x >> 59));
+      x = x * 6364136223846793005ull + 1442695040888963407ull;
+      base[32 * n++] = static_cast<R>(out >> 8) * static_cast<R>(1.0 / 16777216.0);
+    }
+    state[32 * kPoolWords + 32] = static_cast<int>(x);
+    state[32 * kPoolWords + 64] = static_cast<int>(x >> 32);
+  }
+};
+
+// Where word q (1..97) of a seeded state goes in the warp form: the value
+// of lane `lane` `age` steps ago.
+__host__ __device__ inline void pool_place(int q, int *age, int *lane) {
+  *age = q <= 96 ? (q - 1) / 32 + 1 : 4;
+  *lane = q <= 96 ? 32 * *age - q : 31;
+}
+// Weyl term of lane l before its first number.
+__host__ __device__ inline int pool_weyl(int l) {
+  long long c = (kWeylStart - (l + 1ll) * kWeylStep + kWeylStep32) % kWeylMod;
+  return static_cast<int>(c < 0 ? c + kWeylMod : c);
 }
 
 }  // namespace omcgpu

@@ -27,8 +27,11 @@ using omc::fail;
 namespace {
 
 constexpr int kBlock = 128;  // lanes per block
-// Shared memory of a block: the RANMAR states of its lanes, 3 bytes a word.
+// Shared memory of a block: per-lane schedule, the RANMAR states of its
+// lanes, 3 bytes a word; wavefront, the lanes' stacks of random numbers.
 constexpr size_t kRngSmem = static_cast<size_t>(RNG_WORDS) * kBlock * 3;
+template <typename R>
+constexpr size_t kPoolSmem = static_cast<size_t>(kBlock) * (kPoolSlots * sizeof(R) + kPoolState * sizeof(int));
 // Blocks per SM the register budget is sized for, measured on the 6 MV
 // slab.  Wavefront kernel, with electrons near a boundary in their own
 // queue (before the photon flight cap): FP32 5 blocks (96 registers)
@@ -77,6 +80,25 @@ __global__ void seed_kernel(int ixx, int jxx, int nlanes, int *rng_u, int *rng_i
   rng_ijc[2 * nlanes + lane] = 362436;
 }
 
+// Warp streams of the wavefront schedule, from stream `first` on, in the
+// form of RngPool.
+__global__ void seed_pool_kernel(int ixx, int jxx, long long first, int nlanes, int *rng_w) {
+  const int warp = blockIdx.x * blockDim.x + threadIdx.x;
+  if (warp >= nlanes / 32) return;
+  int ik, jk, u[RNG_WORDS];
+  stream_seeds(ixx, jxx, first + warp, &ik, &jk);
+  ranmar_seed(ik, jk, u, 1);
+  for (int l = 0; l < 32; l++) {
+    rng_w[3 * nlanes + warp * 32 + l] = 0;
+    rng_w[4 * nlanes + warp * 32 + l] = pool_weyl(l);
+  }
+  for (int q = 1; q <= RNG_WORDS; q++) {
+    int age, l;
+    pool_place(q, &age, &l);
+    rng_w[(age - 1) * nlanes + warp * 32 + l] = u[q - 1];
+  }
+}
+
 __global__ void ranmar_draw_kernel(int nlanes, long long n, int *rng_u, int *rng_ijc, int *out) {
   int lane = blockIdx.x * blockDim.x + threadIdx.x;
   if (lane >= nlanes) return;
@@ -122,7 +144,10 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kMinBlocks) transport_ke
   if (lane >= P.nlanes) return;
   RngPlanes sp = rng_planes(s_raw);
   rng_to_smem(P.rng_u, P.nlanes, lane, sp, t);
-  Lane<R, false> L(P, lane, sp.lo + t, sp.hi + t, kBlock);
+  Lane<R, false> L(P, lane);
+  L.rng.lo = sp.lo + t;
+  L.rng.hi = sp.hi + t;
+  L.rng.stride = kBlock;
   L.rng.i = P.rng_ijc[lane];
   L.rng.j = P.rng_ijc[P.nlanes + lane];
   L.rng.c = P.rng_ijc[2 * P.nlanes + lane];
@@ -257,13 +282,15 @@ __device__ __forceinline__ unsigned vload(const unsigned *p) { return *static_ca
 
 template <typename R, bool MULTI, bool HBH = false>
 __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wavefront_kernel(Params<R> P, Wavefront<R> W) {
-  extern __shared__ unsigned char s_raw[];
+  extern __shared__ __align__(16) unsigned char s_raw[];
   const int t = threadIdx.x;
   const int gtid = blockIdx.x * kBlock + t;
   const int lane_id = t & 31;
-  RngPlanes sp = rng_planes(s_raw);
-  rng_to_smem(P.rng_u, P.nlanes, gtid, sp, t);
-  Lane<R, true, MULTI, HBH> L(P, gtid, sp.lo + t, sp.hi + t, kBlock);
+  Lane<R, true, MULTI, HBH> L(P, gtid);
+  L.rng.base = reinterpret_cast<R *>(s_raw) + static_cast<size_t>(t >> 5) * 32 * kPoolSlots + lane_id;
+  L.rng.state = reinterpret_cast<int *>(s_raw + static_cast<size_t>(kBlock) * kPoolSlots * sizeof(R)) +
+                (t >> 5) * 32 * kPoolState + lane_id;
+  L.rng.restore(P.rng_w, P.nlanes, gtid);
   if constexpr (HBH) {
     // Each warp's table for merging a completed history's deposits.
     __shared__ int s_hir[kBlock / 32][kHbhRegions];
@@ -271,9 +298,6 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
     L.hbh_tir = s_hir[t >> 5];
     L.hbh_tx = s_hx[t >> 5];
   }
-  L.rng.i = P.rng_ijc[gtid];
-  L.rng.j = P.rng_ijc[P.nlanes + gtid];
-  L.rng.c = P.rng_ijc[2 * P.nlanes + gtid];
   // Photon and discrete electron interactions run in their own chunks
   // (measured on the 6 MV slab: electrons FP32 2.85e7 -> 3.10e7 and FP64
   // 2.02e6 -> 2.22e6 hist/s; photons then 3.96e7 -> 4.29e7).
@@ -355,6 +379,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
       if (lane_id == 0) base = atomicAdd(W.work + cin * (kCounterPad / 2), 32ull);
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base >= total) break;
+      L.rng.refill();
       const unsigned long long i = base + lane_id;
       if (base >= r_in && base < r_ph) {
         const unsigned long long k = i - r_in;
@@ -382,26 +407,32 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
         // A chunk lies in one of the two electron ranges.
         const bool nb = base >= r_eb;
         const unsigned long long k = i - (nb ? r_eb : r_el);
-        if (k < (nb ? n_eb : n_el)) {
-          // Up to chunk_events iterations of electron()'s tstep loop on
-          // this electron; it goes back to a queue if it is still alive
-          // (or if an interaction left a photon on top), to the
-          // interaction queue if its step ended at a deferred interaction.
-          // In the drain the interaction runs at once and the take goes on
-          // with whatever electron is left on top.
-          L.take(QUEUE_EL, bin, nb ? P.q.cap - 1 - static_cast<unsigned>(k) : static_cast<unsigned>(k));
-          L.pending_interaction = false;
-          int n = 0;
-          do {
+        // Up to chunk_events iterations of electron()'s tstep loop on
+        // this electron; it goes back to a queue if it is still alive
+        // (or if an interaction left a photon on top), to the
+        // interaction queue if its step ended at a deferred interaction.
+        // In the drain the interaction runs at once and the take goes on
+        // with whatever electron is left on top; the warp steps together,
+        // so that its random numbers are topped up before every step.
+        bool go = k < (nb ? n_eb : n_el);
+        if (go) L.take(QUEUE_EL, bin, nb ? P.q.cap - 1 - static_cast<unsigned>(k) : static_cast<unsigned>(k));
+        else L.alive = false;
+        L.pending_interaction = false;
+        const int most = drain ? kDrainSteps : W.chunk_events;
+        for (int n = 1;; n++) {
+          if (go) {
             L.electron_event();
             events++;
             if (drain && L.pending_interaction) {
               L.pending_interaction = false;
               L.deferred_interaction();
             }
-          } while (L.alive && !L.pending_interaction && L.p.iq != 0 && ++n < (drain ? kDrainSteps : W.chunk_events));
-          if (L.alive) L.dest = L.pending_interaction ? QUEUE_EI : L.step_queue();
+            go = L.alive && !L.pending_interaction && L.p.iq != 0;
+          }
+          if (n >= most || !__any_sync(0xffffffffu, go)) break;
+          L.rng.refill();
         }
+        if (L.alive) L.dest = L.pending_interaction ? QUEUE_EI : L.step_queue();
       } else {
         const unsigned long long k = i - r_ei;
         if (k < n_ei) {
@@ -425,10 +456,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
     if (!bar_ok) L.err |= ERR_BARRIER;
   }
   if (it >= W.max_iters) L.err |= ERR_LOOP;
-  rng_from_smem(P.rng_u, P.nlanes, gtid, sp, t);
-  P.rng_ijc[gtid] = L.rng.i;
-  P.rng_ijc[P.nlanes + gtid] = L.rng.j;
-  P.rng_ijc[2 * P.nlanes + gtid] = L.rng.c;
+  L.rng.save(P.rng_w, P.nlanes, gtid);
   atomicAdd(P.ensrc, L.ensrc);
   atomicAdd(P.events, events);
   atomicAdd(P.n_geom, L.n_geom);
@@ -719,9 +747,11 @@ struct omc_engine {
   PrecisionState<float> f32;
   // geometry scalars
   int nreg = 0;
-  // per-lane RNG state
-  DevBuf rng_u, rng_ijc;
-  int seeded_lanes = 0;  // lane count the current streams were seeded for
+  // RANMAR state: per-lane streams (rng_u, rng_ijc), or the wavefront
+  // schedule's warp streams (rng_w)
+  DevBuf rng_u, rng_ijc, rng_w;
+  int seeded_lanes = 0;     // lane count the current streams were seeded for
+  bool seeded_wf = false;   // ... in the wavefront schedule's form
   // tallies and counters
   DevBuf endep, acc, acc2, counters, wf_counters;
   // voxel densities (FP64) for the dose conversion of beamlet jobs
@@ -1084,7 +1114,7 @@ struct WfCounters {
 
 template <typename R, bool MULTI = false, bool HBH = false>
 int wavefront_blocks(omc_engine *e) {
-  size_t smem = kRngSmem;
+  size_t smem = kPoolSmem<R>;
   cudaFuncSetAttribute(wavefront_kernel<R, MULTI, HBH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        static_cast<int>(smem));
   int per_sm = 0;
@@ -1173,6 +1203,7 @@ omc_status run_wavefront(omc_engine *e, PrecisionState<R> &S, const omc_run_conf
   P.next = &dc->next;
   P.rng_u = static_cast<int *>(e->rng_u.p);
   P.rng_ijc = static_cast<int *>(e->rng_ijc.p);
+  P.rng_w = static_cast<int *>(e->rng_w.p);
   P.endep = static_cast<double *>(e->endep.p);
   P.ensrc = &dc->ensrc;
   P.events = &dc->events;
@@ -1211,7 +1242,7 @@ omc_status run_wavefront(omc_engine *e, PrecisionState<R> &S, const omc_run_conf
     W.hbh_reserve = 4ull * nlanes;
   }
   const int nlaunch = job ? 1 : cfg->nbatch;
-  size_t smem = kRngSmem;
+  size_t smem = kPoolSmem<R>;
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
@@ -1332,6 +1363,7 @@ extern "C" void omc_engine_destroy(omc_engine *e) {
   e->f32.key.release();
   e->rng_u.release();
   e->rng_ijc.release();
+  e->rng_w.release();
   e->endep.release();
   e->acc.release();
   e->acc2.release();
@@ -1480,6 +1512,34 @@ static omc_status run_batches_one_launch(omc_engine *e, const omc_run_config *cf
   return s;
 }
 
+// RANMAR streams of a run, seeded unless the run continues the last one's:
+// one per lane or (wavefront) one per warp.  A run that continues streams of
+// the other schedule takes the streams after those.
+static omc_status seed_streams(omc_engine *e, const omc_run_config *cfg, int nlanes, bool wavefront) {
+  const size_t lane_bytes = static_cast<size_t>(nlanes) * sizeof(int);
+  omc_status s;
+  const bool live = cfg->continue_streams && e->seeded_lanes == nlanes;
+  if (live && e->seeded_wf == wavefront) return OMC_OK;
+  e->seeded_lanes = 0;
+  const long long first = live ? nlanes : 0;
+  if (wavefront) {
+    const int warps = nlanes / 32;
+    if ((s = e->rng_w.ensure(kPoolWords * lane_bytes)) != OMC_OK) return s;
+    seed_pool_kernel<<<(warps + 31) / 32, 32, 0, e->stream>>>(cfg->ixx, cfg->jxx, first, nlanes,
+                                                            static_cast<int *>(e->rng_w.p));
+  } else {
+    if ((s = e->rng_u.ensure(RNG_WORDS * lane_bytes)) != OMC_OK) return s;
+    if ((s = e->rng_ijc.ensure(3 * lane_bytes)) != OMC_OK) return s;
+    int ixx = cfg->ixx, jxx = cfg->jxx;
+    if (first > 0) stream_seeds(cfg->ixx, cfg->jxx, first, &ixx, &jxx);
+    seed_kernel<<<(nlanes + 255) / 256, 256, 0, e->stream>>>(ixx, jxx, nlanes, static_cast<int *>(e->rng_u.p),
+                                                            static_cast<int *>(e->rng_ijc.p));
+  }
+  e->seeded_lanes = nlanes;
+  e->seeded_wf = wavefront;
+  return OMC_OK;
+}
+
 // Shared start of every run: validation, schedule and lane count, RANMAR
 // streams (seeded unless continued).
 struct RunPlan {
@@ -1508,17 +1568,7 @@ static omc_status prepare_run(omc_engine *e, const omc_run_config *cfg, RunPlan 
   else rp.nlanes = cfg->nlanes > 0 ? cfg->nlanes : (rp.fp64 ? default_lanes<double>(e) : default_lanes<float>(e));
   rp.depth = cfg->stack_depth > 0 ? cfg->stack_depth : kDefaultDepth + 4 * std::max(1, cfg->nsplit);
   const int nlanes = rp.nlanes;
-  // RANMAR streams, one per lane, seeded for this run.
-  size_t rng_bytes = static_cast<size_t>(RNG_WORDS) * nlanes * sizeof(int);
-  if (e->rng_u.n < rng_bytes) e->seeded_lanes = 0;  // reallocated: streams must be seeded
-  if ((s = e->rng_u.ensure(rng_bytes)) != OMC_OK) return s;
-  if ((s = e->rng_ijc.ensure(static_cast<size_t>(3) * nlanes * sizeof(int))) != OMC_OK) return s;
-  if (!(cfg->continue_streams && e->seeded_lanes == nlanes)) {
-    seed_kernel<<<(nlanes + 255) / 256, 256, 0, e->stream>>>(cfg->ixx, cfg->jxx, nlanes,
-                                                            static_cast<int *>(e->rng_u.p),
-                                                            static_cast<int *>(e->rng_ijc.p));
-    e->seeded_lanes = nlanes;
-  }
+  if ((s = seed_streams(e, cfg, nlanes, rp.wavefront)) != OMC_OK) return s;
   return OMC_OK;
 }
 
@@ -1934,16 +1984,7 @@ omc_status job_round(omc_engine *e, PrecisionState<R> &S, omc_job *const *jobs, 
                      const omc_run_config *cfg, omc_run_stats *stats) {
   const int nlanes = wavefront_blocks<R, true>(e) * kBlock;
   omc_status s;
-  size_t rng_bytes = static_cast<size_t>(RNG_WORDS) * nlanes * sizeof(int);
-  if (e->rng_u.n < rng_bytes) e->seeded_lanes = 0;
-  if ((s = e->rng_u.ensure(rng_bytes)) != OMC_OK) return s;
-  if ((s = e->rng_ijc.ensure(static_cast<size_t>(3) * nlanes * sizeof(int))) != OMC_OK) return s;
-  if (!(cfg->continue_streams && e->seeded_lanes == nlanes)) {
-    seed_kernel<<<(nlanes + 255) / 256, 256, 0, e->stream>>>(cfg->ixx, cfg->jxx, nlanes,
-                                                            static_cast<int *>(e->rng_u.p),
-                                                            static_cast<int *>(e->rng_ijc.p));
-    e->seeded_lanes = nlanes;
-  }
+  if ((s = seed_streams(e, cfg, nlanes, true)) != OMC_OK) return s;
   std::vector<JobSlot<R>> slots(n);
   std::vector<long long> first(n + 1, 0);
   for (int i = 0; i < n; i++) {

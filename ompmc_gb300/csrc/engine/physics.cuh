@@ -17,6 +17,8 @@
 //    phase of the persistent kernel picks it up.
 #pragma once
 
+#include <type_traits>
+
 #include "device.cuh"
 
 namespace omcgpu {
@@ -69,7 +71,7 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 template <typename R, bool WF, bool MULTI = false, bool HBH = false>
 struct Lane {
   const Params<R> &P;
-  Ranmar rng;
+  std::conditional_t<WF, RngPool<R>, Ranmar> rng;
   int lane;
   int slot;  // tally slot of the current history / particle (beamlet jobs;
              // multi-job launches: the job slot)
@@ -106,11 +108,7 @@ struct Lane {
   double *hbh_tx = nullptr;
   unsigned long long hbh_merged = 0, hbh_split = 0;
 
-  __device__ Lane(const Params<R> &prm, int ln, unsigned short *slo, unsigned char *shi, int sstride)
-      : P(prm), lane(ln) {
-    rng.lo = slo;
-    rng.hi = shi;
-    rng.stride = sstride;
+  __device__ Lane(const Params<R> &prm, int ln) : P(prm), lane(ln) {
     np = -1;
     slot = 0;
     batch = 0;
@@ -124,7 +122,28 @@ struct Lane {
     queue_hwm = 0;
   }
 
-  __device__ __forceinline__ R rnd() { return static_cast<R>(rng.next_int()) * RC(1.0 / 16777216.0); }
+  __device__ __forceinline__ R rnd() {
+    if constexpr (WF) {
+#ifdef OMC_POOL_CHECK
+      if (rng.n <= 0) err |= ERR_EVENTS;  // a need() is missing or too small
+#endif
+      rng.n = max(rng.n - 1, 0);
+      return rng.base[32 * rng.n];
+    } else {
+      return static_cast<R>(rng.next_int()) * RC(1.0 / 16777216.0);
+    }
+  }
+  // Wavefront: the next k draws find numbers on the lane's stack.
+  __device__ __forceinline__ void need(int k) {
+    if constexpr (WF) {
+      if (rng.n < k) rng.overflow();
+    }
+  }
+  // A number the reference draws and does not use: only where the order of
+  // the stream counts.
+  __device__ __forceinline__ void skip_rnd() {
+    if constexpr (!WF) (void)rnd();
+  }
 
   // Geometry and source of the current particle: the launch's, or its
   // job's in a multi-job launch.
@@ -646,7 +665,17 @@ struct Lane {
     R A, B, C, cosphi, sinphi;
   };
 
+  // cos and sin of a uniform azimuth.  The reference's box method accepts
+  // pi/4 of its pairs, so a warp ran on until the unluckiest of its lanes
+  // was through (3.3 rounds of two draws on average, 1.3 for a lane); the
+  // wavefront path takes the angle itself from one draw.
   __device__ void azimuth(R &cphi, R &sphi) {
+    if constexpr (WF) {
+      const R t = RC(2) * rnd();
+      if constexpr (sizeof(R) == 4) sincospif(t, &sphi, &cphi);
+      else sincospi(t, &sphi, &cphi);
+      return;
+    }
     R xphi, xphi2, yphi, yphi2, rhophi2;
     int guard = 0;
     do {
@@ -851,6 +880,7 @@ struct Lane {
       R fw, rnno3;
       int guard = 0;
       do {
+        need(3);
         rnno3 = rnd();
         q.x = rnno3 * s.xsize + s.xinl;
         rnno3 = rnd();
