@@ -69,9 +69,20 @@ struct alignas(4 * sizeof(R)) V4 {
 //   el_rg  [q][m][l] = {blcce1, blcce0, range_ep, e_array}
 //   el_q   [q][m][l] = {q1c1, q1c0, q2c1, q2c0}
 //   el_ib  [m][l] = {ebr11, ebr10, pbr11, pbr10},  el_ib2 [m][l] = {pbr21, pbr20, 0, 0}
+// Everything an electron step reads of its energy bin: one cache line in
+// FP32, two in FP64.
+template <typename R>
+struct alignas(16 * sizeof(R)) ElBin {
+  V4<R> sd, te, rg, q;  // as el_sd, el_te, el_rg, el_q
+};
+
 template <typename R>
 struct Tables {
   const V4<R> *ph_mfp, *ph_br, *el_sd, *el_te, *el_rg, *el_q, *el_ib, *el_ib2;
+  // wavefront electron steps: one record per bin and per medium
+  const ElBin<R> *el_bin;  // [q][m][l]
+  const V4<R> *med;        // [m][3] {eke1, eke0, 1/eke1, e_array[0]}, {blcc, xcc, xcc/blcc, te},
+                           // {largest sigma per energy loss e-, e+ (-1: monotone), meke - 1, 0}
   int nmed;
   // per medium
   const R *ge0, *ge1, *eke0, *eke1, *xcc, *blcc, *te, *thmoll, *ap;

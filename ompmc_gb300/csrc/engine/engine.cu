@@ -298,10 +298,6 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
     L.hbh_tir = s_hir[t >> 5];
     L.hbh_tx = s_hx[t >> 5];
   }
-  // Photon and discrete electron interactions run in their own chunks
-  // (measured on the 6 MV slab: electrons FP32 2.85e7 -> 3.10e7 and FP64
-  // 2.02e6 -> 2.22e6 hist/s; photons then 3.96e7 -> 4.29e7).
-  L.defer_interactions = true;
   unsigned long long events = 0;
   int it = 0;
   for (; it < W.max_iters; it++) {
@@ -421,7 +417,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
         const int most = drain ? kDrainSteps : W.chunk_events;
         for (int n = 1;; n++) {
           if (go) {
-            L.electron_event();
+            L.wf_electron_event();
             events++;
             if (drain && L.pending_interaction) {
               L.pending_interaction = false;
@@ -912,6 +908,21 @@ omc_status upload_tables(PrecisionState<R> &S, const omc_tables *t) {
     ib[i] = v4(t->ebr11[i], t->ebr10[i], t->pbr11[i], t->pbr10[i]);
     ib2[i] = v4(t->pbr21[i], t->pbr20[i], 0.0, 0.0);
   }
+  std::vector<V4<R>> bins(4 * sd.size()), med(3 * static_cast<size_t>(nmed));
+  for (size_t i = 0; i < sd.size(); i++) {
+    bins[4 * i] = sd[i];
+    bins[4 * i + 1] = te[i];
+    bins[4 * i + 2] = rg[i];
+    bins[4 * i + 3] = qv[i];
+  }
+  for (int m = 0; m < nmed; m++) {
+    med[3 * m] = v4(t->eke1[m], t->eke0[m], 1.0 / t->eke1[m], t->e_array[static_cast<size_t>(m) * MXEKE]);
+    med[3 * m + 1] = v4(t->blcc[m], t->xcc[m], t->xcc[m] / t->blcc[m], t->te[m]);
+    med[3 * m + 2] = v4(t->sig_ismonotone[m] ? -1.0 : t->esig_e[m], t->sig_ismonotone[nmed + m] ? -1.0 : t->psig_e[m],
+                        t->meke[m] - 1, 0.0);
+  }
+  T.el_bin = reinterpret_cast<const ElBin<R> *>(A.put4(bins));
+  T.med = A.put4(med);
   T.el_sd = A.put4(sd);
   T.el_te = A.put4(te);
   T.el_rg = A.put4(rg);

@@ -80,7 +80,6 @@ struct Lane {
   int np;    // top slot, -1 = empty (per-lane schedule)
   Particle<R> p;
   bool alive;           // wavefront: p still needs to be queued
-  bool defer_interactions = false;  // wavefront: queue photon and discrete electron interactions
   bool pending_interaction = false; // wavefront: p ended its step at an interaction
   R skin = 0;           // wavefront: skin depth of p's last step (0: none, or vacuum)
   R cont_mfp = -1;      // wavefront: mean free paths left of the photon emitted (-1: a new flight)
@@ -734,6 +733,7 @@ struct Lane {
 
 #include "photon.inc"
 #include "electron.inc"
+#include "wf_electron.inc"
 
   // ---- source -------------------------------------------------------------
   // Energy and charge of a new history (initHistory's first part, the same
