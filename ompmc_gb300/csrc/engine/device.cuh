@@ -41,6 +41,11 @@ constexpr long long kEventCap = 1ll << 22;
 // A photon flight with no crossing cap (split photons, the per-lane
 // schedule, the end-of-run drain).
 constexpr int kNoFlightCap = 1 << 30;
+// Crossings a wavefront photon flight works out before it looks at them.
+#ifndef OMC_FLIGHT_AHEAD
+#define OMC_FLIGHT_AHEAD 2
+#endif
+constexpr int kFlightAhead = OMC_FLIGHT_AHEAD;
 
 // ---------------------------------------------------------------------------
 // Particles.  dnear is not carried: the reference writes it but never reads
@@ -145,7 +150,7 @@ template <typename R>
 struct Geometry {
   int nx, ny, nz, nxy;
   InvariantDivisor div_nx, div_nxy;  // region decode (omc_dosxyz.c:205-207)
-  const R *xb, *yb, *zb;
+  const R *xb, *yb, *zb;  // in one array, in this order
   // [nreg] voxel records {rhof, medium (-1 vacuum / outside)}: one
   // 8-byte (FP32) or 16-byte (FP64) load per voxel visited
   const VoxelRec<R> *vox;

@@ -949,9 +949,12 @@ omc_status upload_geometry(PrecisionState<R> &S, const omc_phantom *ph, const st
   G.nxy = ph->nx * ph->ny;
   G.div_nx = make_divisor(static_cast<unsigned>(ph->nx));
   G.div_nxy = make_divisor(static_cast<unsigned>(G.nxy));
-  G.xb = A.put(ph->xbounds, ph->nx + 1);
-  G.yb = A.put(ph->ybounds, ph->ny + 1);
-  G.zb = A.put(ph->zbounds, ph->nz + 1);
+  std::vector<double> bounds(ph->xbounds, ph->xbounds + ph->nx + 1);  // one array: see flight_dda()
+  bounds.insert(bounds.end(), ph->ybounds, ph->ybounds + ph->ny + 1);
+  bounds.insert(bounds.end(), ph->zbounds, ph->zbounds + ph->nz + 1);
+  G.xb = A.put(bounds.data(), bounds.size());
+  G.yb = G.xb + ph->nx + 1;
+  G.zb = G.yb + ph->ny + 1;
   G.ecut_m = A.put(ecut_m, nmed + 1);
   G.pcut_m = A.put(pcut_m, nmed + 1);
   std::vector<VoxelRec<R>> vox(med.size());

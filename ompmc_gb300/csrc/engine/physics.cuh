@@ -665,19 +665,19 @@ struct Lane {
   };
 
   // cos and sin of a uniform azimuth.  The reference's box method accepts
-  // pi/4 of its pairs, so a warp ran on until the unluckiest of its lanes
-  // was through (3.3 rounds of two draws on average, 1.3 for a lane); the
-  // wavefront path takes the angle itself from one draw.
+  // pi/4 of its pairs, so a warp runs on until the unluckiest of its lanes
+  // is through (3.3 rounds of two draws on average, 1.3 for a lane).  In
+  // FP32 the wavefront path takes the angle itself from one draw; in FP64
+  // sincospi would cost 2.5 times the FP64 instructions of the rounds.
   __device__ void azimuth(R &cphi, R &sphi) {
-    if constexpr (WF) {
-      const R t = RC(2) * rnd();
-      if constexpr (sizeof(R) == 4) sincospif(t, &sphi, &cphi);
-      else sincospi(t, &sphi, &cphi);
+    if constexpr (WF && sizeof(R) == 4) {
+      sincospif(RC(2) * rnd(), &sphi, &cphi);
       return;
     }
     R xphi, xphi2, yphi, yphi2, rhophi2;
     int guard = 0;
     do {
+      need(2);
       xphi = rnd();
       xphi = RC(2) * xphi - RC(1);
       xphi2 = xphi * xphi;
