@@ -298,7 +298,10 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
     L.hbh_tir = s_hir[t >> 5];
     L.hbh_tx = s_hx[t >> 5];
   }
-  unsigned long long events = 0;
+  __shared__ double s_src[kBlock];
+  s_src[t] = 0.0;
+  L.src_e = s_src + t;
+  unsigned events = 0, hwm = 0;
   int it = 0;
   for (; it < W.max_iters; it++) {
     const int bin = it & 1, bout = bin ^ 1;
@@ -316,6 +319,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
     if (gtid == 0 && static_cast<unsigned long long>(vload(queue_ctr(P.q.ctr, QUEUE_EL, cin))) + vload(queue_ctr(P.q.ctr, QUEUE_EB, cin)) > P.q.cap)
       L.err |= ERR_QUEUE;
     const unsigned long long injected = *static_cast<volatile unsigned long long *>(W.injected + bin);
+    if (gtid == 0) hwm = max(hwm, max(max(n_ph, n_pi), max(max(n_el, n_ei), n_eb)));
     const long long remaining = P.nhist - static_cast<long long>(injected);
     const unsigned long long inflight = static_cast<unsigned long long>(n_ph) + n_el + n_ei + n_pi + n_eb;
     if (W.trace && gtid == 0 && it < W.trace_cap) {
@@ -453,11 +457,11 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
   }
   if (it >= W.max_iters) L.err |= ERR_LOOP;
   L.rng.save(P.rng_w, P.nlanes, gtid);
-  atomicAdd(P.ensrc, L.ensrc);
-  atomicAdd(P.events, events);
-  atomicAdd(P.n_geom, L.n_geom);
-  atomicAdd(P.n_dep, L.n_dep);
-  atomicMax(W.hwm, L.queue_hwm);
+  atomicAdd(P.ensrc, s_src[t]);
+  atomicAdd(P.events, static_cast<unsigned long long>(events));
+  atomicAdd(P.n_geom, static_cast<unsigned long long>(L.n_geom));
+  atomicAdd(P.n_dep, static_cast<unsigned long long>(L.n_dep));
+  if (gtid == 0) *W.hwm = hwm > 0 ? hwm - 1 : 0;
   if constexpr (HBH) {
     if (L.hbh_merged) atomicAdd(P.hbh.histories, L.hbh_merged);
     if (L.hbh_split) atomicAdd(P.hbh.split, L.hbh_split);

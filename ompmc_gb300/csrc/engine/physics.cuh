@@ -88,12 +88,15 @@ struct Lane {
   int gen = 0;          // wavefront: generation and counter slot this phase
   int slot_out = 0;     // appends to
   int dest = QUEUE_NONE;  // wavefront: queue p goes to at the end of the event
-  unsigned queue_hwm;   // highest slot appended
-  double ensrc;
+  double ensrc;         // per-lane schedule
+  double *src_e = nullptr;  // wavefront: source energy of the lane's histories, in shared memory
   unsigned err;
   int max_np;
-  unsigned long long n_geom;  // howfar calls (voxel-stepping decisions)
-  unsigned long long n_dep;   // ausgab calls (energy deposits)
+  // howfar calls (voxel-stepping decisions) and ausgab calls (energy
+  // deposits) of this lane; 32 bits on the wavefront path, where a lane has
+  // its share of the events of one launch and registers bound the occupancy
+  using Count = std::conditional_t<WF, unsigned, unsigned long long>;
+  Count n_geom, n_dep;
   // history-by-history scoring (HBH): head block of the current particle's
   // history (-1: not tracked), particles emitted by the current take, the
   // ring entries written before this iteration began, a history this lane
@@ -118,7 +121,6 @@ struct Lane {
     n_geom = 0;
     n_dep = 0;
     alive = false;
-    queue_hwm = 0;
   }
 
   __device__ __forceinline__ R rnd() {
@@ -275,7 +277,6 @@ struct Lane {
       err |= ERR_QUEUE;
       return;
     }
-    if (idx > queue_hwm) queue_hwm = idx;
     const bool b = kind == QUEUE_EB;
     store_slot(b ? QUEUE_EL : kind, b ? P.q.cap - 1 - idx : idx, q, mfp);
   }
@@ -766,6 +767,7 @@ struct Lane {
     }
     q.e = (q.iq != 0) ? ein + RC(0.5109989461) : ein;
     if constexpr (MULTI) atomicAdd(js->ensrc, static_cast<double>(ein));
+    else if constexpr (WF) *src_e += static_cast<double>(ein);
     else ensrc += static_cast<double>(ein);
   }
 
