@@ -225,6 +225,13 @@ constexpr int kDefaultChunkEvents = 1;
 constexpr int kDrainPerWarp = 32;
 constexpr int kDrainSteps = 4096;
 
+// Steps of one boundary event (wf_boundary_event()).  6 MV slab (2 mm) at 1 /
+// 2 / 3 / 4 / 6 / 8 steps: FP32 717 / 627 / 610 / 603 / 608 / 618 ms; FP64
+// 908 / 912 / 912 / 928 / 962 / 995 ms, the 5x5 cm FP64 job 253 / 243 / 251 /
+// 259 / 262 / 253 ms.  In FP64 a lane that has left the run costs more.
+template <typename R>
+constexpr int kSinglePasses = sizeof(R) == 4 ? 4 : 2;
+
 template <typename R>
 constexpr unsigned long long kInflightPerThread = sizeof(R) == 4 ? 128 : 96;
 
@@ -301,7 +308,8 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
   __shared__ double s_src[kBlock];
   s_src[t] = 0.0;
   L.src_e = s_src + t;
-  unsigned events = 0, hwm = 0;
+  unsigned hwm = 0;
+  L.single_passes = kSinglePasses<R>;
   int it = 0;
   for (; it < W.max_iters; it++) {
     const int bin = it & 1, bout = bin ^ 1;
@@ -393,7 +401,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
         if (k < n_ph) {
           L.take(QUEUE_PH, bin, static_cast<unsigned>(k));
           L.wf_photon_event();
-          events++;
+          L.events++;
         }
       } else if (base >= r_pi && base < r_el) {
         const unsigned long long k = i - r_pi;
@@ -421,8 +429,8 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
         const int most = drain ? kDrainSteps : W.chunk_events;
         for (int n = 1;; n++) {
           if (go) {
-            L.wf_electron_event();
-            events++;
+            if (nb && !drain) L.wf_boundary_event();
+            else L.wf_electron_event();
             if (drain && L.pending_interaction) {
               L.pending_interaction = false;
               L.deferred_interaction();
@@ -458,7 +466,7 @@ __global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wav
   if (it >= W.max_iters) L.err |= ERR_LOOP;
   L.rng.save(P.rng_w, P.nlanes, gtid);
   atomicAdd(P.ensrc, s_src[t]);
-  atomicAdd(P.events, static_cast<unsigned long long>(events));
+  atomicAdd(P.events, static_cast<unsigned long long>(L.events));
   atomicAdd(P.n_geom, static_cast<unsigned long long>(L.n_geom));
   atomicAdd(P.n_dep, static_cast<unsigned long long>(L.n_dep));
   if (gtid == 0) *W.hwm = hwm > 0 ? hwm - 1 : 0;

@@ -81,6 +81,8 @@ struct Lane {
   Particle<R> p;
   bool alive;           // wavefront: p still needs to be queued
   bool pending_interaction = false; // wavefront: p ended its step at an interaction
+  int single_passes = 1;  // wavefront: steps of one boundary event at most
+  unsigned events = 0;  // wavefront: electron steps and photon flights
   R skin = 0;           // wavefront: skin depth of p's last step (0: none, or vacuum)
   R cont_mfp = -1;      // wavefront: mean free paths left of the photon emitted (-1: a new flight)
   R taken_mfp = -1;     // wavefront: mean free paths left of the photon taken (-1: a new flight)
