@@ -32,27 +32,31 @@ constexpr int kBlock = 128;  // lanes per block
 constexpr size_t kRngSmem = static_cast<size_t>(RNG_WORDS) * kBlock * 3;
 template <typename R>
 constexpr size_t kPoolSmem = static_cast<size_t>(kBlock) * (kPoolSlots * sizeof(R) + kPoolState * sizeof(int));
-// Blocks per SM the register budget is sized for, measured on the 6 MV
-// slab.  Wavefront kernel, with electrons near a boundary in their own
-// queue (before the photon flight cap): FP32 5 blocks (96 registers)
-// 8.39e7 hist/s, against 8.23e7 with
-// 4; FP64 2 blocks (248 registers) 7.04e6 at 96 particles per thread in
-// flight, against 6.88e6 with 3 blocks (168 registers) and 6.90e6 with 4
-// (128 registers, 368 bytes of spills) at the same number in flight.
-// Per-lane kernel: 5 and 3.
+// Blocks per SM the register budget is sized for.  FP32 wavefront: 6 blocks
+// (80 registers, about 100 bytes of spills) against 5 (96, none): slab on 1
+// cm voxels 81.6 -> 77.9 ms, dij 85.0 -> 81.3 ms, 250 kVp job 6.3 -> 6.0 ms,
+// 6 MV slab on 2 mm 603 ms both; the server's multi-job kernel loses (144.9
+// -> 150.9 ms) and keeps 5, as does history scoring, whose registers spill
+// more.  FP64 wavefront: 2 blocks (236 registers); 3 (168) measured 3% to 7%
+// slower, its bound is the FP64 pipe.  Per-lane kernel: 5 and 3.
 #ifndef OMC_MIN_BLOCKS_FP32
 #define OMC_MIN_BLOCKS_FP32 5
 #endif
 #ifndef OMC_MIN_BLOCKS_FP64
 #define OMC_MIN_BLOCKS_FP64 3
 #endif
+#ifndef OMC_WF_MIN_BLOCKS_FP32
+#define OMC_WF_MIN_BLOCKS_FP32 6
+#endif
 #ifndef OMC_WF_MIN_BLOCKS_FP64
 #define OMC_WF_MIN_BLOCKS_FP64 2
 #endif
-template <typename R>
+template <typename R, bool PLAIN = true>
 struct Occupancy {
   static constexpr int kMinBlocks = sizeof(R) == 4 ? OMC_MIN_BLOCKS_FP32 : OMC_MIN_BLOCKS_FP64;
-  static constexpr int kWavefrontMinBlocks = sizeof(R) == 4 ? OMC_MIN_BLOCKS_FP32 : OMC_WF_MIN_BLOCKS_FP64;
+  // PLAIN: neither multi-job nor history scoring.
+  static constexpr int kWavefrontMinBlocks =
+      sizeof(R) == 4 ? (PLAIN ? OMC_WF_MIN_BLOCKS_FP32 : OMC_MIN_BLOCKS_FP32) : OMC_WF_MIN_BLOCKS_FP64;
 };
 constexpr int kDefaultDepth = 48;
 // History-by-history block pool: blocks per particle in flight, times 2.
@@ -233,7 +237,7 @@ template <typename R>
 constexpr int kSinglePasses = sizeof(R) == 4 ? 4 : 2;
 
 template <typename R>
-constexpr unsigned long long kInflightPerThread = sizeof(R) == 4 ? 128 : 96;
+constexpr unsigned long long kInflightPerThread = 96;
 
 // Voxel crossings of a photon flight per event (nsplit = 1), measured on the
 // 6 MV slab (hist/s): FP32 9.52e7 / 9.72e7 / 9.63e7 / 9.20e7 at 8 / 16 / 32
@@ -288,7 +292,7 @@ __device__ bool grid_barrier(unsigned *arrive, unsigned *gen, unsigned nblocks,
 __device__ __forceinline__ unsigned vload(const unsigned *p) { return *static_cast<const volatile unsigned *>(p); }
 
 template <typename R, bool MULTI, bool HBH = false>
-__global__ void __launch_bounds__(kBlock, Occupancy<R>::kWavefrontMinBlocks) wavefront_kernel(Params<R> P, Wavefront<R> W) {
+__global__ void __launch_bounds__(kBlock, (Occupancy<R, !MULTI && !HBH>::kWavefrontMinBlocks)) wavefront_kernel(Params<R> P, Wavefront<R> W) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   const int t = threadIdx.x;
   const int gtid = blockIdx.x * kBlock + t;
