@@ -65,7 +65,7 @@ struct alignas(4 * sizeof(R)) V4 {
 // ---------------------------------------------------------------------------
 // Tables resident on the device, converted to R.  Scalar arrays keep the
 // reference's index layout (the arrays of omc_tables); the interpolation
-// coefficients read on every step are also packed per (medium, energy bin)
+// coefficients read on every step are packed per (medium, energy bin)
 // into V4 records so that a lookup is one load:
 //   ph_mfp [m][l] = {gmfp1, gmfp0, cohe1, cohe0}
 //   ph_br  [m][l] = {gbr11, gbr10, gbr21, gbr20}
@@ -93,24 +93,18 @@ struct Tables {
   const R *ge0, *ge1, *eke0, *eke1, *xcc, *blcc, *te, *thmoll, *ap;
   const R *esig_e, *psig_e, *delcm, *zbrang, *bpar0, *bpar1;
   const int *monotone;  // [2*nmed]
-  // photon [nmed*MXGE]
-  const R *gmfp0, *gmfp1, *gbr10, *gbr11, *gbr20, *gbr21, *cohe0, *cohe1, *pmax0, *pmax1;
+  const R *pmax0, *pmax1;  // Rayleigh [nmed*MXGE]
   // rayleigh [MXRAYFF] of medium 0 (see rayleigh())
   const R *xgrid, *fcum, *b_array, *c_array;
   const int *i_array;
   // pair/brems [nmed*8]
   const R *dl1, *dl2, *dl3, *dl4, *dl5, *dl6;
-  // electron [nmed*MXEKE]
-  const R *esig0, *esig1, *psig0, *psig1, *ededx0, *ededx1, *pdedx0, *pdedx1;
-  const R *ebr10, *ebr11, *pbr10, *pbr11, *pbr20, *pbr21, *tmxs0, *tmxs1, *blcce0, *blcce1;
-  const R *etae0, *etae1, *etap0, *etap1, *q1ce0, *q1ce1, *q1cp0, *q1cp1, *q2ce0, *q2ce1, *q2cp0, *q2cp1;
-  const R *e_array, *range_ep;  // range_ep [2*nmed*MXEKE]
   const int *meke;              // [nmed]
   // spin
   R b2spin_min, dbeta2i, espml, dleneri, dqq1i;
   const R *spin_rej;
   // msnew
-  const R *ums, *fms, *wms;
+  const R *ums, *wms;
   const int *ims;
   R dllambi, dqmsi;
 };

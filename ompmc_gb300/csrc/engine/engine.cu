@@ -828,14 +828,6 @@ omc_status upload_tables(PrecisionState<R> &S, const omc_tables *t) {
   T.bpar1 = A.put(t->bpar1, nmed);
   T.monotone = A.put_int(t->sig_ismonotone, 2 * nmed);
   T.meke = A.put_int(t->meke, nmed);
-  T.gmfp0 = A.put(t->gmfp0, ng);
-  T.gmfp1 = A.put(t->gmfp1, ng);
-  T.gbr10 = A.put(t->gbr10, ng);
-  T.gbr11 = A.put(t->gbr11, ng);
-  T.gbr20 = A.put(t->gbr20, ng);
-  T.gbr21 = A.put(t->gbr21, ng);
-  T.cohe0 = A.put(t->cohe0, ng);
-  T.cohe1 = A.put(t->cohe1, ng);
   T.pmax0 = A.put(t->pmax0, ng);
   T.pmax1 = A.put(t->pmax1, ng);
   // Rayleigh sampling reads medium 0's form-factor tables (see rayleigh()).
@@ -850,38 +842,6 @@ omc_status upload_tables(PrecisionState<R> &S, const omc_tables *t) {
   T.dl4 = A.put(t->dl4, 8 * nmed);
   T.dl5 = A.put(t->dl5, 8 * nmed);
   T.dl6 = A.put(t->dl6, 8 * nmed);
-  T.esig0 = A.put(t->esig0, ne);
-  T.esig1 = A.put(t->esig1, ne);
-  T.psig0 = A.put(t->psig0, ne);
-  T.psig1 = A.put(t->psig1, ne);
-  T.ededx0 = A.put(t->ededx0, ne);
-  T.ededx1 = A.put(t->ededx1, ne);
-  T.pdedx0 = A.put(t->pdedx0, ne);
-  T.pdedx1 = A.put(t->pdedx1, ne);
-  T.ebr10 = A.put(t->ebr10, ne);
-  T.ebr11 = A.put(t->ebr11, ne);
-  T.pbr10 = A.put(t->pbr10, ne);
-  T.pbr11 = A.put(t->pbr11, ne);
-  T.pbr20 = A.put(t->pbr20, ne);
-  T.pbr21 = A.put(t->pbr21, ne);
-  T.tmxs0 = A.put(t->tmxs0, ne);
-  T.tmxs1 = A.put(t->tmxs1, ne);
-  T.blcce0 = A.put(t->blcce0, ne);
-  T.blcce1 = A.put(t->blcce1, ne);
-  T.etae0 = A.put(t->etae_ms0, ne);
-  T.etae1 = A.put(t->etae_ms1, ne);
-  T.etap0 = A.put(t->etap_ms0, ne);
-  T.etap1 = A.put(t->etap_ms1, ne);
-  T.q1ce0 = A.put(t->q1ce_ms0, ne);
-  T.q1ce1 = A.put(t->q1ce_ms1, ne);
-  T.q1cp0 = A.put(t->q1cp_ms0, ne);
-  T.q1cp1 = A.put(t->q1cp_ms1, ne);
-  T.q2ce0 = A.put(t->q2ce_ms0, ne);
-  T.q2ce1 = A.put(t->q2ce_ms1, ne);
-  T.q2cp0 = A.put(t->q2cp_ms0, ne);
-  T.q2cp1 = A.put(t->q2cp_ms1, ne);
-  T.e_array = A.put(t->e_array, ne);
-  T.range_ep = A.put(t->range_ep, 2 * ne);
   T.b2spin_min = static_cast<R>(t->b2spin_min);
   T.dbeta2i = static_cast<R>(t->dbeta2i);
   T.espml = static_cast<R>(t->espml);
@@ -889,7 +849,6 @@ omc_status upload_tables(PrecisionState<R> &S, const omc_tables *t) {
   T.dqq1i = static_cast<R>(t->dqq1i);
   T.spin_rej = A.put(t->spin_rej, nspin);
   T.ums = A.put(t->ums, nms);
-  T.fms = A.put(t->fms, nms);
   T.wms = A.put(t->wms, nms);
   T.ims = A.put_int(t->ims, nms);
   T.dllambi = static_cast<R>(t->dllambi);
