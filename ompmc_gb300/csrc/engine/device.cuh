@@ -198,16 +198,17 @@ constexpr int kBatchTag = 4096;
 // adds the history's energy x in each region to sum[r] and x^2 to sum2[r]
 // -- the history-by-history estimators of Walters, Kawrakow and Rogers
 // (Med. Phys. 29 (2002) 2745) -- then returns the blocks.  Blocks of 384
-// bytes: a 16-byte header and (region, energy) entries.
+// bytes: a 20-byte header and (region, energy) entries.
 constexpr int kHbhBlockBytes = 384;
 constexpr int kHbhRegions = 128;  // distinct regions of one history the warp's merge table holds
 template <typename R>
 struct HbhBlock {
-  static constexpr int kEntries = (kHbhBlockBytes - 16) / static_cast<int>(4 + sizeof(R));
+  static constexpr int kEntries = (kHbhBlockBytes - 20) / static_cast<int>(4 + sizeof(R));
   int count;  // entries appended; those past kEntries went to the next block
   int next;   // continuation block, -1 none
   int live;   // head block: particles of the history queued or being processed
   int slot;   // head block: tally slot (batch) of the history
+  int tail;   // head block: a block near the end of the chain (-1: none), see Lane::hbh_append
   int ir[kEntries];
   R x[kEntries];
 };
@@ -247,13 +248,12 @@ struct QueueLayout {
 };
 
 // Every counter of the schedule has an L2 line of its own, kCounterPad words
-// apart.  All warps append to the same few queues, so the counters are the
-// hottest addresses of the run, and one L2 line serves about one atomic per
-// clock: side by side in one line, as they were, they bounded the kernel
-// whatever its occupancy or instruction count.
-// Measured, lines apart against side by side: 6 MV slab (2 mm, 10x10 cm2,
-// 1e8 histories, FP32) 1061 -> 959 ms; a 250 kVp job of 6e6 histories 9.1 ->
-// 7.9 ms; FP64 jobs unchanged within their spread.
+// apart.  All warps append to the same few queues and claim from the same
+// counter, about seven atomics per history on one line as they were laid out
+// (the 46 deposits spread over the tallies), and an L2 line serves its
+// atomics one after another.  Measured, lines apart against side by side: 6
+// MV slab (2 mm, 10x10 cm2, 1e8 histories, FP32) 1061 -> 959 ms; a 250 kVp
+// job of 6e6 histories 9.1 -> 7.9 ms; FP64 jobs unchanged within their spread.
 constexpr int kCounterPad = 64;
 // Counter of queue kind q in rotation slot c (0..2).
 __device__ __forceinline__ unsigned *queue_ctr(unsigned *ctr, int q, int c) { return ctr + (3 * q + c) * kCounterPad; }
