@@ -424,7 +424,8 @@ __host__ __device__ inline void stream_seeds(int ixx, int jxx, long long k, int 
 // adds numbers of a generator of the lane's own (PCG32, O'Neill,
 // HMC-CS-2014-0905), whose state is drawn from the warp's stream at launch.
 // (A call that carried on with a RANMAR stream per lane in device memory cost
-// 100 to 300 bytes of register spills around the call sites.)
+// 72 to 452 bytes of register spills, by kernel and version, around the call
+// sites.)
 // Measured: 6 MV slab (2 mm, 1e8 histories) FP32 942 -> 806 ms, FP64 (1e7)
 // 1499 -> 1441 ms; slab on 1 cm voxels 116 -> 98 ms; positron field 55 -> 44
 // ms; nsplit 16 40 -> 34 ms; dij 116 -> 102 ms.

@@ -37,7 +37,7 @@ constexpr size_t kPoolSmem = static_cast<size_t>(kBlock) * (kPoolSlots * sizeof(
 // cm voxels 81.6 -> 77.9 ms, dij 85.0 -> 81.3 ms, 250 kVp job 6.3 -> 6.0 ms,
 // 6 MV slab on 2 mm 603 ms both; the server's multi-job kernel loses (144.9
 // -> 150.9 ms) and keeps 5, as does history scoring, whose registers spill
-// more.  FP64 wavefront: 2 blocks (236 registers); 3 (168) measured 3% to 7%
+// more.  FP64 wavefront: 2 blocks (234 registers); 3 (168) measured 3% to 7%
 // slower, its bound is the FP64 pipe.  Per-lane kernel: 5 and 3.
 #ifndef OMC_MIN_BLOCKS_FP32
 #define OMC_MIN_BLOCKS_FP32 5
